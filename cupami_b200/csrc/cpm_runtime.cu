@@ -13,6 +13,8 @@
 #include "k_deep.cuh"
 #include "k_local.cuh"
 #include "k_rows.cuh"
+#include "k_cond.cuh"
+#include "k_order.cuh"
 #include "k_apriori.cuh"
 #include "k_periodic.cuh"
 #include "k_costmodel.cuh"
@@ -46,6 +48,8 @@ using namespace cpm;
 #include "rt_database.inc"
 #include "rt_pairs.inc"
 #include "rt_deep.inc"
+#include "rt_cond.inc"
+#include "rt_order.inc"
 #include "rt_eclat.inc"
 #include "rt_apriori.inc"
 #include "rt_periodic.inc"

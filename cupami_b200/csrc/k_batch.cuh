@@ -15,7 +15,10 @@ struct DbDesc {
     const uint64_t *bits;      // item-major tidsets
     const uint32_t *support;   // per column
     uint32_t *freq;            // frequent columns, increasing
-    uint32_t *C;               // F x F pair Gram (upper triangle)
+    uint32_t *fsup;            // their supports
+    const uint32_t *ord;       // mining rank -> frequent index (deep levels extend by increasing rank)
+    const uint32_t *crank;     // frequent column -> mining rank
+    uint32_t *C;               // F x F pair Gram (upper triangle); below it, the pair patterns' ids
     uint64_t stride;           // words per tidset
     uint32_t n_items;
     uint32_t F;                // frequent items (set by the host after compaction)
@@ -44,7 +47,11 @@ __global__ void k_compact_frequent_b(const DbDesc *__restrict__ d, uint32_t *__r
             if (w < wid) before += warp_tot[w];
             total += warp_tot[w];
         }
-        if (pass) D.freq[base + before + __popc(bal & ((1u << lane) - 1))] = c;
+        if (pass) {
+            const uint32_t k = base + before + __popc(bal & ((1u << lane) - 1));
+            D.freq[k] = c;
+            D.fsup[k] = D.support[c];
+        }
         __syncthreads();
         if (threadIdx.x == 0) base += total;
         __syncthreads();
@@ -107,28 +114,45 @@ __device__ __forceinline__ uint32_t db_of_row(const DbDesc *d, uint32_t n_db, ui
     return lo;
 }
 
-// cnt[r] = passing pairs (i, j > i) of global frequent row r; warp per row.
+// cnt[r] = passing pairs (i, j > i) of global frequent row r, sum[r] = their
+// supports added up; ccnt[row_base + a] (zeroed) = members of the class of
+// rank a, its pairs with items of higher rank.  Warp per row.
 __global__ void k_pair_count_b(const DbDesc *__restrict__ d, uint32_t n_db, uint64_t n_rows,
-                               uint32_t *__restrict__ cnt) {
+                               uint32_t *__restrict__ cnt, uint64_t *__restrict__ sum, uint32_t *__restrict__ ccnt) {
     const uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned lane = threadIdx.x & 31;
     if (r >= n_rows) return;
     const DbDesc D = d[db_of_row(d, n_db, r)];
     const uint64_t i = r - D.row_base;
-    uint32_t c = 0;
-    for (uint64_t j = i + 1 + lane; j < D.F; j += 32) c += (long long)D.C[i * D.F + j] >= D.minsup;
+    const uint32_t rank = D.crank[D.freq[i]];
+    uint32_t c = 0, mine = 0;
+    unsigned long long t = 0;
+    for (uint64_t j = i + 1 + lane; j < D.F; j += 32) {
+        const uint32_t s = D.C[i * D.F + j];
+        if ((long long)s >= D.minsup) {
+            ++c;
+            t += s;
+            const uint32_t other = D.crank[D.freq[j]];
+            if (other > rank) ++mine;
+            else atomicAdd(ccnt + D.row_base + other, 1u);
+        }
+    }
     c = warp_sum_u32(c);
-    if (!lane) cnt[r] = c;
+    mine = warp_sum_u32(mine);
+    t = warp_sum_u64(t);
+    if (!lane) {
+        cnt[r] = c;
+        sum[r] = t;
+        if (mine) atomicAdd(ccnt + D.row_base + rank, mine);
+    }
 }
 
-// Singleton and pair patterns plus top-level member tables; warp per global
-// frequent row r.  off[r] = global index of row r's first pair.
+// Singleton and pair patterns; warp per global frequent row r.  off[r] =
+// global index of row r's first pair.  The pair's id goes below C's diagonal.
 __global__ void k_emit_b(const DbDesc *__restrict__ d, uint32_t n_db, uint64_t n_rows,
                          const uint64_t *__restrict__ off, uint32_t *__restrict__ pat_parent,
                          uint32_t *__restrict__ pat_item, uint32_t *__restrict__ pat_sup,
-                         uint32_t *__restrict__ pat_db, uint32_t *__restrict__ mem_pat,
-                         uint32_t *__restrict__ mem_item, const uint64_t **__restrict__ mem_bits,
-                         const unsigned long long *__restrict__ row_list) {
+                         uint32_t *__restrict__ pat_db) {
     const uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned lane = threadIdx.x & 31;
     if (r >= n_rows) return;
@@ -157,7 +181,35 @@ __global__ void k_emit_b(const DbDesc *__restrict__ d, uint32_t n_db, uint64_t n
             pat_item[pid] = item;
             pat_sup[pid] = s;
             if (pat_db) pat_db[pid] = db;
-            mem_pat[k] = (uint32_t)pid;
+            D.C[j * D.F + i] = (uint32_t)pid;
+        }
+        pos += __popc(bal);
+    }
+}
+
+// Member tables of the top-level classes: the class of rank a holds the items
+// of higher rank whose pair with it passed, in rank order, at coff[row_base +
+// a].  Warp per class, after k_emit_b.
+__global__ void k_class_b(const DbDesc *__restrict__ d, uint32_t n_db, uint64_t n_rows,
+                          const uint64_t *__restrict__ coff, uint32_t *__restrict__ mem_pat,
+                          uint32_t *__restrict__ mem_item, const uint64_t **__restrict__ mem_bits,
+                          const unsigned long long *__restrict__ row_list) {
+    const uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned lane = threadIdx.x & 31;
+    if (r >= n_rows) return;
+    const DbDesc D = d[db_of_row(d, n_db, r)];
+    const uint64_t a = r - D.row_base, i = D.ord[a];
+    uint64_t pos = coff[r];
+    for (uint64_t b0 = a + 1; b0 < D.F; b0 += 32) {
+        const uint64_t b = b0 + lane;
+        const uint64_t j = b < D.F ? D.ord[b] : i;
+        const uint64_t lo = min(i, j), hi = max(i, j);
+        const bool pass = b < D.F && (long long)D.C[lo * D.F + hi] >= D.minsup;
+        const unsigned bal = __ballot_sync(CPM_FULL, pass);
+        if (pass) {
+            const uint64_t k = pos + __popc(bal & ((1u << lane) - 1));
+            const uint32_t item = D.freq[j];
+            mem_pat[k] = D.C[hi * D.F + lo];
             mem_item[k] = item;
             // The item's transaction-id list where one was built (bit 0 set), else its bitset.
             const unsigned long long lp = row_list ? row_list[D.row_base + j] : 0ull;

@@ -72,6 +72,8 @@ struct DFrame {
     // `stride` words, member q at bits + q * stride.  Their transactions are
     // numbered by rank within the tidset of the unit that made the frame.
     const uint64_t *bits = nullptr;
+    uint32_t used = 0;  // 16-byte words of the `stride` that hold transactions (0: all)
+    uint32_t pad = 0;
 };
 
 // Every counter that CTAs update or poll sits on its own 128-byte line, so
@@ -96,6 +98,7 @@ struct DeepState {
     CPM_LINE(lq_pending);   // projected units queued or running
     CPM_LINE(local_units);  // projected units run
     CPM_LINE(h_units);      // row-wise units run
+    CPM_LINE(n_cframes);    // frames of conditional rows (k_cond)
     unsigned int error;
     unsigned int pad[31];
 };

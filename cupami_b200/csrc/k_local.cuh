@@ -77,7 +77,7 @@ __device__ int local_claim(const DeepParams &P, unsigned long long *item) {
 struct LocalUnit {
     const ulonglong2 *base;  // member 0's tidset
     uint64_t mem_off;
-    uint32_t m, p, w2, root, db;
+    uint32_t m, p, w2, pitch, root, db;  // a tidset: w2 16-byte words, pitch from the last
     long long minsup;
 };
 
@@ -174,8 +174,8 @@ __device__ __forceinline__ void local_unit(const DeepParams &P, const LocalUnit 
     const uint32_t lg = W2 >= 32 ? 5u : (W2 <= 1 ? 0u : 32u - (uint32_t)__clz(W2 - 1u));
     const uint32_t G = 1u << lg, NG = 32u >> lg, gi = lane >> lg, gl = lane & (G - 1u);
     const uint32_t cnt = u.m - u.p - 1;
-    const ulonglong2 *pre2 = u.base + (uint64_t)u.p * W2;
-    const ulonglong2 *sib0 = pre2 + W2;  // later member q (from 0) at sib0 + q * W2
+    const ulonglong2 *pre2 = u.base + (uint64_t)u.p * u.pitch;
+    const ulonglong2 *sib0 = pre2 + u.pitch;  // later member q (from 0) at sib0 + q * pitch
     const ulonglong2 zero = make_ulonglong2(0ull, 0ull);
     // The prefix, staged in this warp's slot of shared memory.
     for (uint32_t j = lane; j < W2; j += 32) s_pre[j] = ld_cg(pre2 + j);
@@ -191,7 +191,7 @@ __device__ __forceinline__ void local_unit(const DeepParams &P, const LocalUnit 
 #pragma unroll
             for (int k = 0; k < K; ++k) {
                 const uint32_t j = gl + G * k;
-                x[v][k] = (q < cnt && j < W2) ? ld_cg(sib0 + (uint64_t)q * W2 + j) : zero;
+                x[v][k] = (q < cnt && j < W2) ? ld_cg(sib0 + (uint64_t)q * u.pitch + j) : zero;
             }
         }
     };
@@ -289,13 +289,13 @@ __device__ __forceinline__ void local_unit_wide(const DeepParams &P, const Local
                                              LocalCounters &cs) {
     DeepState *st = P.st;
     const uint32_t W2 = u.w2, cnt = u.m - u.p - 1;
-    const ulonglong2 *pre2 = u.base + (uint64_t)u.p * W2;
-    const ulonglong2 *sib0 = pre2 + W2;
+    const ulonglong2 *pre2 = u.base + (uint64_t)u.p * u.pitch;
+    const ulonglong2 *sib0 = pre2 + u.pitch;
     const ulonglong2 zero = make_ulonglong2(0ull, 0ull);
     const uint32_t parent_pat = __ldcg(P.mem_pat + u.mem_off + u.p);
     const uint64_t item_off = u.mem_off + u.p + 1;
     auto count = [&](uint32_t q) {
-        const ulonglong2 *sb = sib0 + (uint64_t)q * W2;
+        const ulonglong2 *sb = sib0 + (uint64_t)q * u.pitch;
         uint32_t c = 0;
         for (uint32_t j0 = 0; j0 < W2; j0 += 128) {
             ulonglong2 a[4], b[4];
@@ -349,7 +349,7 @@ __device__ __forceinline__ void local_unit_wide(const DeepParams &P, const Local
     for (uint32_t q = 0; q < cnt && run < ns; ++q) {
         const uint32_t c = count(q);
         if ((long long)c < u.minsup) continue;
-        const ulonglong2 *sb = sib0 + (uint64_t)q * W2;
+        const ulonglong2 *sb = sib0 + (uint64_t)q * u.pitch;
         ulonglong2 *o = out + (uint64_t)run * W2;
         for (uint32_t j = lane; j < W2; j += 32) o[j] = and2(ld_cg(sb + j), ld_cg(pre2 + j));
         if (lane == 0) local_emit(P, u, parent_pat, __ldcg(P.mem_item + item_off + q), c, pid0 + run, mb, run, o);
@@ -389,11 +389,13 @@ __global__ void __launch_bounds__(LOCAL_BLOCK, 4) k_local(DeepParams P) {
         u.mem_off = __ldcg(reinterpret_cast<const unsigned long long *>(&fp->mem_off));
         u.m = __ldcg(&fp->m);
         u.p = (uint32_t)item;
-        u.w2 = __ldcg(&fp->stride) / 2u;
+        u.pitch = __ldcg(&fp->stride) / 2u;
+        u.w2 = __ldcg(&fp->used);
+        if (!u.w2) u.w2 = u.pitch;
         u.root = __ldcg(&fp->root);
         u.db = __ldcg(&fp->db);
         u.minsup = __ldcg(&fp->minsup);
-        if (!u.base || u.w2 == 0 || u.w2 > (LOCAL_MAX_BITS + 127) / 128 || u.p + 1 >= u.m) {
+        if (!u.base || u.w2 == 0 || u.w2 > u.pitch || u.pitch > (LOCAL_MAX_BITS + 127) / 128 || u.p + 1 >= u.m) {
             if (lane == 0) deep_fail(st, DEEP_ERR_INTERNAL);
             break;
         }

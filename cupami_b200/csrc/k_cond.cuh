@@ -20,7 +20,7 @@
 //
 // The top frame of a database is its rows of frequent indices (k_cond_top);
 // its units build the classes of the pair level, whose supports the Gram
-// already holds.  Child frames whose bitsets are small (ns members of
+// already holds (or which k_cond_count itself counted).  Child frames whose bitsets are small (ns members of
 // ceil(R / 128) 16-byte words each, at most bitset_work in all) are written as
 // bitsets over the kept rows and mined by k_local, a warp per unit; larger
 // ones stay rows.  Few do: below the classes of rare items everything is
@@ -512,6 +512,11 @@ __device__ __forceinline__ void cond_map(const CondParams &P, const CBig &u, con
     for (uint32_t r = threadIdx.x; r < u.ns; r += COND_BLOCK) sm[crank[P.d.mem_item[u.mb + r]] - p1] = r;
 }
 
+// Supports of every unit's later members, into the pool -- or, for units of a
+// top frame, the pairs of their item, into the Gram matrix (zeroed): sparse
+// databases count their pairs this way instead of multiplying tidsets
+// (1M x 20k, 4,612 frequent items: pair level 3.0 ms, 1.1 of it the rows that the
+// deep levels need anyway, against 13.5 ms on the tensor cores).
 __global__ void __launch_bounds__(COND_BLOCK, 3) k_cond_count(CondParams P) {
     extern __shared__ uint32_t sm[];
     const unsigned long long chunks = min(P.now.n[1], (unsigned long long)P.chunks_cap);
@@ -525,9 +530,19 @@ __global__ void __launch_bounds__(COND_BLOCK, 3) k_cond_count(CondParams P) {
         __syncthreads();
         cond_count(f.idx, f.occ + u.start + a, n, f.lg, p1, sm, lc);
         __syncthreads();
-        for (uint32_t q = threadIdx.x; q < cnt; q += COND_BLOCK) {
-            const uint32_t s = cond_copies_sum(sm, q, lc);
-            if (s) atomicAdd(P.pool + u.pool + q, s);
+        if (f.top) {
+            const DbDesc &d = P.dbs[f.db];
+            const uint64_t i = d.ord[u.p];
+            for (uint32_t q = threadIdx.x; q < cnt; q += COND_BLOCK) {
+                const uint32_t s = cond_copies_sum(sm, q, lc);
+                const uint64_t j = d.ord[p1 + q];
+                if (s) atomicAdd(d.C + min(i, j) * d.F + max(i, j), s);
+            }
+        } else {
+            for (uint32_t q = threadIdx.x; q < cnt; q += COND_BLOCK) {
+                const uint32_t s = cond_copies_sum(sm, q, lc);
+                if (s) atomicAdd(P.pool + u.pool + q, s);
+            }
         }
         __syncthreads();
     }

@@ -132,11 +132,17 @@ __global__ void k_count_pruned(const uint64_t *__restrict__ bits, uint64_t strid
 // candidates joined on left row a of the level (t in [poff[a], poff[a] +
 // partners[a]), cand rows L[a] + one last item) share the k items of L[a], so
 // their complete intersection is (AND of the k rows of L[a]) AND (the last
-// item's row).  One CTA takes one left row at a time (grid stride): it stages
-// the prefix AND in shared memory once (stride words), then each warp streams
-// one candidate's last-item row against it, eight 16-byte loads in flight per
-// lane.  A group of p candidates reads k + p rows instead of (k + 1) p.
+// item's row).  One CTA takes one left row, or one of up to COUNT_PARTS equal
+// shares of its candidates when it has more than COUNT_SHARE (grid stride): it
+// stages the prefix AND in shared memory once (stride words; not where pruning
+// left no candidate), then each warp streams one candidate's last-item row
+// against it, eight 16-byte loads in flight per lane.  Without the shares the
+// CTA of the row with the most partners (over a hundred, against three on
+// average) ended alone: planted 100k x 1,000, 43.6 -> 37.6, 44.1 -> 35.7, 17.5 -> 22.7
+// and 13.3 -> 14.1 us on its levels, at about 7.5 TB/s of L2.  (Equal blocks of candidates instead of
+// left rows stage a prefix every few candidates: 89 us.)
 // *bytes_alg gains the rows read.  Rows at or past *d_n have no partners.
+constexpr uint32_t COUNT_PARTS = 8, COUNT_SHARE = 16;
 __global__ void __launch_bounds__(256) k_count_grouped(const uint64_t *__restrict__ bits, uint64_t stride,
                                                        const uint32_t *__restrict__ L, const uint64_t *__restrict__ d_n,
                                                        uint32_t k, const uint64_t *__restrict__ poff,
@@ -150,9 +156,23 @@ __global__ void __launch_bounds__(256) k_count_grouped(const uint64_t *__restric
     const uint64_t n = *d_n, n2 = stride / 2;
     const uint32_t w = k + 1;
     unsigned long long rows_read = 0;
-    for (uint64_t a = blockIdx.x; a < n; a += gridDim.x) {
-        const uint32_t p = partners[a];
-        if (!p) continue;  // the same for every thread of the CTA
+    for (uint64_t x = blockIdx.x; x < n * COUNT_PARTS; x += gridDim.x) {
+        const uint64_t a = x % n;
+        const uint32_t part = (uint32_t)(x / n), p = partners[a];
+        const uint32_t parts = min(COUNT_PARTS, (p + COUNT_SHARE - 1) / COUNT_SHARE);
+        if (part >= parts) continue;  // the same for every thread of the CTA
+        const uint64_t t0 = poff[a] + (uint64_t)p * part / parts, t1 = poff[a] + (uint64_t)p * (part + 1) / parts;
+        bool alive = false;
+        for (uint64_t t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
+            if (ok_flag[t]) {
+                alive = true;
+            } else {
+                support[t] = 0;
+                pass[t] = 0;
+            }
+        }
+        // (also the barrier between the last reads of the prefix and this one's writes)
+        if (!__syncthreads_or(alive)) continue;
         const uint32_t *ra = L + a * k;
         for (uint64_t v = threadIdx.x; v < n2; v += blockDim.x) {
             ulonglong2 acc = ld_stream(reinterpret_cast<const ulonglong2 *>(bits + (uint64_t)ra[0] * stride) + v);
@@ -161,25 +181,17 @@ __global__ void __launch_bounds__(256) k_count_grouped(const uint64_t *__restric
             s_pre[v] = acc;
         }
         __syncthreads();
-        const uint64_t t0 = poff[a];
-        for (uint32_t j = wid; j < p; j += nw) {
-            const uint64_t t = t0 + j;
-            if (!ok_flag[t]) {
-                if (!lane) {
-                    support[t] = 0;
-                    pass[t] = 0;
-                }
-                continue;
-            }
+        for (uint64_t t = t0 + wid; t < t1; t += nw) {
+            if (!ok_flag[t]) continue;
             const ulonglong2 *row = reinterpret_cast<const ulonglong2 *>(bits + (uint64_t)cand[t * w + k] * stride);
             uint32_t s = 0;
             uint64_t v = lane;
             for (; v + 224 < n2; v += 256) {
-                ulonglong2 x[8];
+                ulonglong2 y[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) x[u] = ld_stream(row + v + 32 * u);
+                for (int u = 0; u < 8; ++u) y[u] = ld_stream(row + v + 32 * u);
 #pragma unroll
-                for (int u = 0; u < 8; ++u) s += popc2(and2(x[u], s_pre[v + 32 * u]));
+                for (int u = 0; u < 8; ++u) s += popc2(and2(y[u], s_pre[v + 32 * u]));
             }
             for (; v < n2; v += 32) s += popc2(and2(ld_stream(row + v), s_pre[v]));
             s = warp_sum_u32(s);
@@ -190,7 +202,6 @@ __global__ void __launch_bounds__(256) k_count_grouped(const uint64_t *__restric
             }
         }
         if (!threadIdx.x) rows_read += k;  // the prefix rows
-        __syncthreads();
     }
     if (!lane && rows_read) atomicAdd(bytes_alg, rows_read * 8ull * stride);
 }

@@ -118,6 +118,8 @@ _SIGNATURES = {
     "cpm_result_trace": (ctypes.c_int, [_P, _P, _P, ctypes.POINTER(_U64)]),
     "cpm_tdb_from_csr": (ctypes.c_int, [_P, _P, _U64, _P, _U64, ctypes.c_uint32, _P, ctypes.c_int64,
                                         ctypes.POINTER(_P)]),
+    "cpm_tdb_from_ids": (ctypes.c_int, [_P, _P, _U64, _P, _U64, _P, ctypes.c_int64, ctypes.POINTER(_P)]),
+    "cpm_count_rows": (ctypes.c_int, [_P, _U64, ctypes.POINTER(_U64)]),
     "cpm_mine_periodic": (ctypes.c_int, [_P, _P, ctypes.c_int64, ctypes.c_int64, ctypes.c_int, ctypes.POINTER(_P)]),
     "cpm_result_copy_periodic": (ctypes.c_int, [_P, ctypes.c_int, _P, _P, _P, _P]),
     "cpm_result_from_tree_periodic": (ctypes.c_int, [_P, _P, _P, _P, _U64, ctypes.POINTER(_P)]),
@@ -297,6 +299,22 @@ class Database:
                                                  ctypes.byref(handle)))
         return cls(ctx, handle)
 
+    @classmethod
+    def from_temporal_ids(cls, ctx, offsets, ids, timestamps, end):
+        """from_temporal over raw integer ids (``labels``: the id of every column)."""
+        offsets = np.ascontiguousarray(offsets, dtype=np.uint64)
+        ids = np.ascontiguousarray(ids, dtype=np.uint32)
+        timestamps = np.ascontiguousarray(timestamps, dtype=np.int64)
+        handle = _P()
+        with ctx.lock:
+            ctx.check(library().cpm_tdb_from_ids(ctx.handle, _ptr(offsets), offsets.size - 1, _ptr(ids), ids.size,
+                                                 _ptr(timestamps), int(end), ctypes.byref(handle)))
+        db = cls(ctx, handle)
+        db.labels = np.zeros(db.n_items, dtype=np.uint32)
+        if db.n_items:
+            ctx.check(library().cpm_db_labels(handle, db.labels.ctypes.data))
+        return db
+
     def mine_periodic(self, min_sup, max_per, algorithm, order):
         """Periodic-frequent itemsets of a temporal database (Result with ``periods``)."""
         res = _P()
@@ -332,6 +350,17 @@ class Database:
             self.close()
         except Exception:
             pass
+
+
+def count_rows(offsets):
+    """Rows of a CSR (uint64 offsets) that hold items."""
+    if offsets.size < 2:
+        return 0
+    if offsets.size <= 1 << 14 or not LIB_PATH.exists():
+        return int(np.count_nonzero(offsets[1:] > offsets[:-1]))
+    n = _U64()
+    library().cpm_count_rows(offsets.ctypes.data, offsets.size - 1, ctypes.byref(n))
+    return n.value
 
 
 def join_labels(offsets, items, labels, sep="\t"):

@@ -168,7 +168,7 @@ class cuApriori:
         offsets = np.ascontiguousarray(offsets, dtype=np.uint64)
         ids = np.ascontiguousarray(ids, dtype=np.uint32)
         self._csr = (offsets, ids)
-        self._transactionCount = int(np.count_nonzero(offsets[1:] > offsets[:-1]))
+        self._transactionCount = _native.count_rows(offsets)
         previous = self._inputBackend.get("reason")
         self._inputBackend = {"backend": backend, "reason": reason}
         if previous and backend == "numpy-cuda":

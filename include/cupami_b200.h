@@ -171,6 +171,9 @@ int cpm_db_from_ids_batch(cpm_ctx *ctx, uint32_t n_db, const uint64_t *const *of
 int cpm_autotune(cpm_ctx *ctx, cpm_db *db, int64_t min_sup, const cpm_opts *opts,
                  int32_t *block, int32_t *ctas_per_sm, int32_t *list_div, double *ms_deep);
 
+/* Rows of a CSR that hold items (the transaction count behind fractional
+ * thresholds, cuApriori.py:452-456).  Host only. */
+int  cpm_count_rows(const uint64_t *offsets, uint64_t n_rows, uint64_t *n_nonempty);
 int  cpm_db_info(const cpm_db *db, uint64_t *n_transactions, uint32_t *n_items,
                  uint64_t *words);
 int  cpm_db_labels(const cpm_db *db, uint32_t *ids_out);  /* n_items entries */
@@ -263,6 +266,10 @@ void *cpm_stream(const cpm_ctx *ctx);
  * nondecreasing; end >= the last timestamp.  Every column must be < n_items. */
 int cpm_tdb_from_csr(cpm_ctx *ctx, const uint64_t *offsets, uint64_t n_rows, const uint32_t *cols,
                      uint64_t nnz, uint32_t n_items, const int64_t *timestamps, int64_t end, cpm_db **out);
+/* The same from raw integer ids, as cpm_db_from_ids: distinct ids ordered as
+ * their decimal strings sort, cpm_db_labels() returns them in column order. */
+int cpm_tdb_from_ids(cpm_ctx *ctx, const uint64_t *offsets, uint64_t n_rows, const uint32_t *ids,
+                     uint64_t nnz, const int64_t *timestamps, int64_t end, cpm_db **out);
 /* Itemsets with support >= min_sup, support > 0 and periodicity <= max_per
  * (_temporal.py:166-171).  algo CPM_ECLAT (cuPFEclat) or CPM_APRIORI
  * (cuPFApriori): the same itemsets; copy them with cpm_result_copy_periodic in

@@ -97,6 +97,7 @@ struct DeepState {
     CPM_LINE(lq_tail);      // projected units: entries reserved
     CPM_LINE(lq_pending);   // projected units queued or running
     CPM_LINE(local_units);  // projected units run
+    CPM_LINE(local_frames); // child frames that the warps of k_local kept to themselves
     CPM_LINE(h_units);      // row-wise units run
     CPM_LINE(n_cframes);    // frames of conditional rows (k_cond)
     unsigned int error;

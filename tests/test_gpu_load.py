@@ -44,7 +44,8 @@ def test_temporal_ids_match_the_oracle(n, items, step):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("step", [1, 1 << 23])  # ids of 2**26 and more: one database after the other
+# Presence bitmaps in shared memory, in device memory; ids of 2**26 and more: one database after the other.
+@pytest.mark.parametrize("step", [1, 1 << 14, 1 << 23])
 def test_batch_of_uneven_databases(oracle_lib, step):
     from cupami_b200 import TransactionCSR, cuEclat
 

@@ -894,8 +894,8 @@ def run_ours(args, world, rank, local):
         # The last collective: rank 0's baselines below run on its own, so no
         # rank waits on a barrier while they do.
         pg.destroy_process_group()
-    # Roofline of the deep phase (k_deep, then k_local for the units below
-    # projected prefixes), the step's dominant part on Eclat workloads, from
+    # Roofline of the deep phase (conditional rows or k_deep, then k_local for
+    # the units below small prefixes), the step's dominant part on Eclat workloads, from
     # its own CUDA events.
     hbm, bf16, src = peaks()
     eclat_stats = [[st for a, st, _ in out if a != "apriori"] for out in per_kernel]
@@ -908,9 +908,11 @@ def run_ours(args, world, rank, local):
         row_units = statistics.mean(sum(s.get("row_units", 0) for s in st) for st in eclat_stats)
         units = statistics.mean(sum(s.get("work_items", 0) for s in st) for st in eclat_stats)
         achieved = deep_bytes / (deep_ms * 1e-3) / 1e9 if deep_ms else 0.0
-        tr = deep_traffic(args.workload, args.tidsets, args.arena_mb)
+        # The committed record is of the tidset walk; pairs counted from the rows mean the other engine ran.
+        tr = deep_traffic(args.workload, args.tidsets, args.arena_mb) if all(
+            s["pair_ops"] for st in eclat_stats for s in st) else None
         traffic = tr["dram_bytes_per_launch"] if tr else None
-        roof = {"kernel": "deep phase: k_deep (persistent, a CTA per unit) then k_local (a warp per projected unit)",
+        roof = {"kernel": "deep phase: conditional rows (k_cond_*) or k_deep, then k_local (a warp per projected unit)",
                 "bound": deep_bound(traffic, deep_bytes),
                 "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm, "traffic": traffic,
                 "peak_source": src, "frac_of": "HBM copy bandwidth (" + src + "); algorithmic bytes / kernel time",
@@ -925,7 +927,7 @@ def run_ours(args, world, rank, local):
                 "units": units, "projected_units": proj_units, "row_units": row_units,
                 "alg_bytes": "sum over units of the prefix, every sibling and every child written, each at its "
                              "own form's size (bitset 8*W, list 16 + 4*ids, projected bitset 16*ceil(n/128)); "
-                             "row-wise units count their prefix's rows instead of the siblings (12 B per row "
+                             "units counted row by row: their prefix's rows instead of the siblings (12 B per row "
                              "+ 2 B per frequent index)"}
     pair_ms = statistics.mean(sum(st["ms_pairs"] for _, st, _ in out) for out in per_kernel)
     pair_ops = statistics.mean(sum(st["pair_ops"] for _, st, _ in out) for out in per_kernel)

@@ -97,6 +97,9 @@ class cuApriori:
     #: (1-4); 0 leaves each to the library (or to the autotuner's table).
     _DEEP_BLOCK = 0
     _DEEP_CTAS_PER_SM = 0
+    #: (With these and the deep-level options below all 0, larger searches are
+    #: mined in order of support over conditional rows; any of them set selects
+    #: the walk over tidsets that they describe.)
     #: Tidset forms of the deep levels: 0 automatic (bitsets, plus transaction-id
     #: lists for sparse tidsets of databases too big for the L2); 1 bitsets
     #: only; 2 lists wherever possible.

@@ -14,7 +14,7 @@
  *   cpm_mine(algo = CPM_APRIORI)
  *       replaces cuApriori.mine + _generateCandidates + _countCandidateSupports
  *       (cupami/frequentPattern/cuApriori.py:473-535)
- *   cpm_tdb_from_csr + cpm_mine_periodic
+ *   cpm_tdb_from_csr / cpm_tdb_from_ids + cpm_mine_periodic
  *       replace TemporalInput._prepare + cuPFEclat.mine / cuPFApriori.mine
  *       (cupami/periodicFrequentPattern/_temporal.py:150-171,
  *        cuPFEclat.py:146-175, cuPFApriori.py:141-157)
@@ -65,7 +65,7 @@ extern "C" {
 /* Pattern order produced by cpm_result_copy. */
 #define CPM_ORDER_ECLAT    0  /* insertion order of cuEclat.mine (cuEclat.py:168-245) */
 #define CPM_ORDER_APRIORI  1  /* insertion order of cuApriori.mine: by length, then tuple */
-#define CPM_ORDER_NONE     2  /* device emission order (fastest) */
+#define CPM_ORDER_NONE     2  /* whatever order the search left them in (fastest) */
 #define CPM_ORDER_DEPTH_FIRST 3  /* insertion order of cuPFEclat.mine: singletons, then for each
                                     pattern in depth-first order its extensions
                                     (cupami/periodicFrequentPattern/cuPFEclat.py:150-173) */
@@ -89,6 +89,9 @@ typedef struct {
     int32_t  deep_block;           /* deep-level kernel threads per CTA: 128, 256, 512 or 1024; 0 = automatic */
     int32_t  deep_ctas_per_sm;     /* resident deep-level CTAs per SM, 1-4 (capped by occupancy); 0 = automatic */
     int32_t  autotune;             /* 1: use the launch shape cpm_autotune found for this tidset length */
+    /* With tidsets, list_div, deep_*, arena_bytes and collect_trace all 0, searches of some size are
+       mined in order of increasing support over conditional rows; what follows is then the walk over
+       tidsets of the others (any option set selects that walk, in column order). */
     int32_t  tidsets;              /* deep-level tidset forms.  0: bitsets, plus transaction-id lists for
                                       tidsets held by under 1/32 of the transactions when a database's
                                       frequent bitsets exceed half the L2 and one bitset fits in shared
@@ -115,7 +118,8 @@ typedef struct {
     uint64_t work_items;           /* (frame, position) units processed */
     uint64_t intersections;        /* sibling AND+popcount operations */
     uint64_t bytes_alg;            /* sum over units of 8*W*(1 + siblings + survivors) */
-    uint64_t pair_ops;             /* tensor ops issued by the pair Gram (2*K*rows*cols) */
+    uint64_t pair_ops;             /* tensor ops issued by the pair Gram (2*K*rows*cols; 0: pairs counted
+                                      on CUDA cores or from the rows) */
     uint64_t kernel_launches;
     uint64_t retries;              /* arena/queue overflow retries (failed rounds included) */
     uint64_t deep_rounds;          /* memory-bounded rounds of the deep phase (0: one launch) */
@@ -127,7 +131,7 @@ typedef struct {
     double   pair_tops;            /* pair_ops / ms_pairs */
     uint64_t projected_units;      /* of work_items: units below a projected prefix (one warp each) */
     double   ms_local;             /* of ms_deep: the launches that mine those units */
-    uint64_t row_units;            /* of work_items: units counted row by row (deep_rows) */
+    uint64_t row_units;            /* of work_items: units counted row by row (deep_rows, conditional rows) */
 } cpm_stats;
 
 /* ---- context ------------------------------------------------------------ */

@@ -63,6 +63,10 @@ class Opts(ctypes.Structure):
     ]
 
 
+class Limits(ctypes.Structure):
+    _fields_ = [("arena_bytes", ctypes.c_uint64)]
+
+
 class Stats(ctypes.Structure):
     _fields_ = [(n, ctypes.c_uint64) for n in (
         "n_patterns", "n_frequent_items", "n_frequent_pairs", "frames", "work_items",
@@ -82,6 +86,7 @@ _SIGNATURES = {
     "cpm_shutdown": (None, [_P]),
     "cpm_last_error": (ctypes.c_char_p, [_P]),
     "cpm_version": (ctypes.c_char_p, []),
+    "cpm_set_limits": (ctypes.c_int, [_P, _P]),
     "cpm_default_opts": (ctypes.c_int, [ctypes.POINTER(Opts)]),
     "cpm_db_from_csr": (ctypes.c_int, [_P, _P, _U64, _P, _U64, ctypes.c_uint32, ctypes.POINTER(_P)]),
     "cpm_db_from_ids": (ctypes.c_int, [_P, _P, _U64, _P, _U64, ctypes.POINTER(_P)]),
@@ -178,6 +183,11 @@ class Context:
         self.device = device
         self.lock = threading.Lock()
         self.databases = weakref.WeakSet()  # freed before the context (they point to it)
+
+    def set_limits(self, **limits):
+        """cpm_set_limits: what the searches may take (fields of ``Limits``; none: automatic)."""
+        with self.lock:
+            self.check(library().cpm_set_limits(self.handle, ctypes.byref(Limits(**limits))))
 
     def check(self, code):
         if code != CPM_OK:

@@ -134,12 +134,19 @@ typedef struct {
     uint64_t row_units;            /* of work_items: units counted row by row (deep_rows, conditional rows) */
 } cpm_stats;
 
+/* What a context's searches may take, with the engine still chosen automatically (an option of
+ * cpm_opts selects one).  All 0: automatic. */
+typedef struct {
+    uint64_t arena_bytes;          /* child tidsets or conditional rows of one launch */
+} cpm_limits;
+
 /* ---- context ------------------------------------------------------------ */
 int         cpm_init(int device, cpm_ctx **out);
 void        cpm_shutdown(cpm_ctx *ctx);
 const char *cpm_last_error(const cpm_ctx *ctx);
 const char *cpm_version(void);
 int         cpm_default_opts(cpm_opts *opts);
+int         cpm_set_limits(cpm_ctx *ctx, const cpm_limits *limits);  /* NULL: none */
 
 /* ---- databases ------------------------------------------------------------ */
 /* CSR of item columns.  Empty rows are dropped and the rest renumbered in

@@ -1,0 +1,83 @@
+"""GPU: searches under limits that leave the engine automatic, against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def limits():
+    from cupami_b200 import _native
+
+    ctx = _native.context(0)
+    yield ctx.set_limits
+    ctx.set_limits()
+
+
+def _csr(n, items, mean, block=0):
+    """Zipf baskets; ``block`` more items held together by 40 baskets."""
+    from cupami_b200 import TransactionCSR
+
+    rng = np.random.default_rng(n + items)
+    w = 1.0 / np.arange(1, items + 1) ** 0.9
+    held = rng.random((n, items + block)) < np.append(np.minimum(0.97, w * mean / w.sum()), np.zeros(block))
+    held[rng.choice(n, 40, replace=False), items:] = True
+    offsets = np.zeros(n + 1, dtype=np.uint64)
+    np.cumsum(held.sum(axis=1), out=offsets[1:])
+    return TransactionCSR(offsets, np.nonzero(held)[1].astype(np.uint32), items + block)
+
+
+class _Mines:
+    """Mines of one database through the C ABI, each checked against the oracle."""
+
+    def __init__(self, oracle_lib, csr, minsup):
+        from cupami_b200 import _native
+
+        self.minsup, self.csr = minsup, csr
+        self.want = list(oracle_lib.to_dict(*oracle_lib.mine_csr(csr.offsets, csr.items, minsup)).items())
+        self.db = _native.Database.from_ids(_native.context(0), csr.offsets, csr.items)
+
+    def again(self, **opts):
+        from cupami_b200 import _native
+
+        o = _native.Opts()
+        _native.library().cpm_default_opts(o)
+        for name, value in opts.items():
+            setattr(o, name, value)
+        r = self.db.mine(self.minsup, _native.CPM_ECLAT, o)
+        keys = _native.join_labels(r.offsets, r.items, self.db.labels)
+        assert list(zip(keys, r.supports.tolist())) == self.want
+        return r.stats
+
+
+# Steps of less than the fifth that remembered sizes add: one of the budgets is filled to over
+# four fifths, and those below overflow (frames of bitsets alone, and frames of rows).
+@pytest.mark.parametrize("n,items,mean,minsup,most,least", [(20000, 2500, 12, 30, 8 << 20, 176 << 10),
+                                                            (400000, 200, 20, 4000, 1300 << 20, 48 << 20)])
+def test_mines_of_one_database_under_shrinking_arenas(oracle_lib, limits, n, items, mean, minsup, most, least):
+    mines = _Mines(oracle_lib, _csr(n, items, mean), minsup)
+    stats = []
+    while most > least:
+        limits(arena_bytes=most)
+        stats += [mines.again(), mines.again()]
+        most = most * 6 // 7
+    assert stats[0]["retries"] == 0 and stats[0]["deep_rounds"] == 0
+    assert any(s["retries"] for s in stats) and (n < 400000 or any(s["deep_rounds"] for s in stats))
+
+
+def test_a_search_that_overflows_both_engines_is_mined_again(oracle_lib, limits):
+    """Rows, then tidsets, overflow the same arena; the next mines go in rounds from the start."""
+    limits(arena_bytes=64 << 20)
+    mines = _Mines(oracle_lib, _csr(400001, 200, 20), 4000)
+    first, *rest = [mines.again() for _ in range(3)]
+    assert first["retries"] >= 1 and all(s["deep_rounds"] > 0 for s in (first, *rest))
+
+
+def test_a_walk_over_tidsets_does_not_steer_conditional_rows(oracle_lib, limits):
+    mines = _Mines(oracle_lib, _csr(131073, 90, 4), 150)
+    free = mines.again()
+    limits(arena_bytes=4 << 20)
+    walk = mines.again(deep_project=1)  # overflows, goes in rounds
+    assert walk["deep_rounds"] > 0
+    limits()
+    assert mines.again()["deep_rounds"] == 0 and free["deep_rounds"] == 0

@@ -1,4 +1,4 @@
-"""GPU: searches under limits that leave the engine automatic, against the oracle."""
+"""GPU: searches at the edges of the engines' tables and limits, against the oracle."""
 import numpy as np
 import pytest
 
@@ -81,3 +81,29 @@ def test_a_walk_over_tidsets_does_not_steer_conditional_rows(oracle_lib, limits)
     assert walk["deep_rounds"] > 0
     limits()
     assert mines.again()["deep_rounds"] == 0 and free["deep_rounds"] == 0
+
+
+# Thresholds that itemsets of no transaction pass: baskets of one item (frames without a row below
+# the classes), two items that occur among eleven that do not, and a database without transactions.
+@pytest.mark.parametrize("minsup", [0, -3])
+@pytest.mark.parametrize("kind", ["single", "pair", "none"])
+def test_levels_whose_units_have_no_occurrences(kind, minsup):
+    from cupami_b200 import _native
+
+    items, n = 13, 0 if kind == "none" else 1_900_000
+    rng = np.random.default_rng(items)
+    held = np.zeros((n, items), bool)
+    if kind == "single":
+        held[np.arange(n), rng.integers(0, items, n)] = True
+    elif kind == "pair":
+        held[:, [4, 9]] = rng.random((n, 2)) < 0.5
+        held[~held.any(axis=1), 4] = True
+    offsets = np.zeros(n + 1, dtype=np.uint64)
+    np.cumsum(held.sum(axis=1), out=offsets[1:])
+    db = _native.Database.from_columns(_native.context(0), offsets, np.nonzero(held)[1], items)
+    r = db.mine(minsup, _native.CPM_ECLAT)
+    got = {tuple(r.items[r.offsets[k]:r.offsets[k + 1]].tolist()): s for k, s in enumerate(r.supports.tolist())}
+    assert len(got) == len(r) == 2**items - 1
+    occur = {(i,): int(held[:, i].sum()) for i in range(items)}
+    occur[4, 9] = int((held[:, 4] & held[:, 9]).sum())
+    assert all(s == occur.get(p, 0) for p, s in got.items())

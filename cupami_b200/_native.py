@@ -64,7 +64,7 @@ class Opts(ctypes.Structure):
 
 
 class Limits(ctypes.Structure):
-    _fields_ = [("arena_bytes", ctypes.c_uint64)]
+    _fields_ = [(n, ctypes.c_uint64) for n in ("arena_bytes", "level_units")]
 
 
 class Stats(ctypes.Structure):

@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(COND_BLOCK) k_cond_publish(CondParams P) {
                 const unsigned long long k = atomicAdd(P.next.n, 1ull), pc = atomicAdd(P.next.n + 1, (unsigned long long)parts),
                                          pw = atomicAdd(P.next.n + 2, (unsigned long long)cnt);
                 if (k >= P.units_cap || pc + parts > P.chunks_cap || pw + cnt > P.pool_cap) {
-                    deep_fail(st, DEEP_ERR_FRAMES);
+                    deep_fail(st, DEEP_ERR_LEVEL);
                 } else {
                     CBig b;
                     b.fid = (uint32_t)u.frame;

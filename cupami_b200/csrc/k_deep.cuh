@@ -39,6 +39,7 @@ namespace cpm {
 enum : unsigned {
     DEEP_ERR_QUEUE = 1u, DEEP_ERR_ARENA = 2u, DEEP_ERR_MEMBERS = 4u, DEEP_ERR_FRAMES = 8u,
     DEEP_ERR_PATTERNS = 16u, DEEP_ERR_SPIN = 32u, DEEP_ERR_INTERNAL = 64u,
+    DEEP_ERR_LEVEL = 128u,  // a level of conditional rows has more units, chunks or counters than its tables
 };
 
 // 64-bit words of a list of n transaction ids (16-byte header, 16-byte padding).

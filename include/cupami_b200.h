@@ -138,6 +138,7 @@ typedef struct {
  * cpm_opts selects one).  All 0: automatic. */
 typedef struct {
     uint64_t arena_bytes;          /* child tidsets or conditional rows of one launch */
+    uint64_t level_units;          /* units that a level of conditional rows has room for at first */
 } cpm_limits;
 
 /* ---- context ------------------------------------------------------------ */

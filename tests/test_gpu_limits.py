@@ -83,6 +83,16 @@ def test_a_walk_over_tidsets_does_not_steer_conditional_rows(oracle_lib, limits)
     assert mines.again()["deep_rounds"] == 0 and free["deep_rounds"] == 0
 
 
+@pytest.mark.parametrize("units", [1, 40, 100])
+def test_levels_outgrow_their_tables(oracle_lib, limits, units):
+    mines = _Mines(oracle_lib, _csr(400002, 200, 20), 4000)
+    free = mines.again()
+    limits(level_units=units)
+    stats = [mines.again(), mines.again()]
+    assert free["row_units"] > 0 and free["retries"] == 0
+    assert all(s["retries"] > 0 and s["row_units"] == free["row_units"] for s in stats)
+
+
 # Thresholds that itemsets of no transaction pass: baskets of one item (frames without a row below
 # the classes), two items that occur among eleven that do not, and a database without transactions.
 @pytest.mark.parametrize("minsup", [0, -3])

@@ -93,6 +93,24 @@ def test_levels_outgrow_their_tables(oracle_lib, limits, units):
     assert all(s["retries"] > 0 and s["row_units"] == free["row_units"] for s in stats)
 
 
+# No room for the conditional rows (their occurrences take 12 MB); the tables of a search with
+# them (frames: 9.0 MB); the counters of their levels (2 GB).  Each time there is for the walk.
+@pytest.mark.parametrize("shape,limit", [
+    ((400003, 60, 4, 20000), {"arena_bytes": 8 << 20, "alloc_bytes": 8 << 20}),
+    ((20000, 2500, 12, 30), {"arena_bytes": 8 << 20, "alloc_bytes": 17 << 19}),
+    ((400003, 200, 20, 4000), {"arena_bytes": 1 << 30, "alloc_bytes": 1200 << 20, "level_units": 1 << 20})])
+def test_searches_go_on_without_the_memory_they_were_planned_with(oracle_lib, limits, shape, limit):
+    n, items, mean, minsup = shape
+    mines = _Mines(oracle_lib, _csr(n, items, mean), minsup)
+    free = mines.again()
+    limits(**limit)
+    tight = mines.again()
+    limits()
+    again = mines.again()
+    ran = [(s["pair_ops"], s["row_units"], s["bytes_alg"]) for s in (free, tight, again)]  # differ by engine
+    assert ran[0] == ran[2] != ran[1]
+
+
 # Thresholds that itemsets of no transaction pass: baskets of one item (frames without a row below
 # the classes), two items that occur among eleven that do not, and a database without transactions.
 @pytest.mark.parametrize("minsup", [0, -3])

@@ -111,6 +111,24 @@ def test_searches_go_on_without_the_memory_they_were_planned_with(oracle_lib, li
     assert ran[0] == ran[2] != ran[1]
 
 
+def test_blocks_that_fit_only_as_asked_for(oracle_lib, limits):
+    """The tidsets' block is allocated in a size rounded up, or, without room for that, its own."""
+    from cupami_b200 import _native
+
+    csr = _csr(400004, 200, 3)
+    baskets = int(np.count_nonzero(np.diff(csr.offsets.astype(np.int64))))
+    bits = 200 * (-(-baskets // 128) * 2) * 8
+    limits(alloc_bytes=bits - 1)
+    with pytest.raises(_native.NativeError) as e:
+        _Mines(oracle_lib, csr, 8000)
+    assert e.value.code == _native.CPM_ENOMEM
+    limits(alloc_bytes=bits)
+    mines = _Mines(oracle_lib, csr, 8000)
+    assert mines.db.n_items == 200
+    limits()
+    mines.again()
+
+
 # Thresholds that itemsets of no transaction pass: baskets of one item (frames without a row below
 # the classes), two items that occur among eleven that do not, and a database without transactions.
 @pytest.mark.parametrize("minsup", [0, -3])

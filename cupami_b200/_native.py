@@ -64,7 +64,7 @@ class Opts(ctypes.Structure):
 
 
 class Limits(ctypes.Structure):
-    _fields_ = [(n, ctypes.c_uint64) for n in ("arena_bytes", "level_units", "alloc_bytes")]
+    _fields_ = [(n, ctypes.c_uint64) for n in ("arena_bytes", "level_units", "order_bytes", "alloc_bytes")]
 
 
 class Stats(ctypes.Structure):

@@ -56,7 +56,7 @@ struct OrdParams {
 
 // The value of an item (database d): the SplitMix64 output function (Steele,
 // Lea, Flood, "Fast splittable pseudorandom number generators", 2014).
-__device__ __forceinline__ uint64_t ord_value(uint32_t item, uint32_t d) {
+__host__ __device__ __forceinline__ uint64_t ord_value(uint32_t item, uint32_t d) {
     uint64_t z = (((uint64_t)d << 32) | item) + 0x9e3779b97f4a7c15ull;
     z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
     z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;

@@ -139,6 +139,8 @@ typedef struct {
 typedef struct {
     uint64_t arena_bytes;          /* child tidsets or conditional rows of one launch */
     uint64_t level_units;          /* units that a level of conditional rows has room for at first */
+    uint64_t order_bytes;          /* ordering patterns on the device: results that take more are ordered by
+                                      the host */
     uint64_t alloc_bytes;          /* largest block of device memory; one above it ends as one that the
                                       device has no room for */
 } cpm_limits;

@@ -129,6 +129,35 @@ def test_blocks_that_fit_only_as_asked_for(oracle_lib, limits):
     mines.again()
 
 
+# A thousand to half a million patterns, a chain of twelve levels among them, without room on the device
+# to order them; every order of the C ABI.
+@pytest.mark.parametrize("shape", [(131073, 90, 4, 150, 0), (70001, 600, 60, 7000, 0), (20001, 800, 8, 40, 12)])
+def test_patterns_ordered_by_the_host(oracle_lib, limits, shape):
+    from cupami_b200 import _native
+
+    n, items, mean, minsup, block = shape
+    mines = _Mines(oracle_lib, _csr(n, items, mean, block), minsup)
+    orders = (_native.CPM_ORDER_ECLAT, _native.CPM_ORDER_APRIORI, _native.CPM_ORDER_NONE)
+    free = [mines.db.mine(minsup, _native.CPM_ECLAT, order=o) for o in orders]
+    limits(order_bytes=1)
+    mines.again()
+    tight = [mines.db.mine(minsup, _native.CPM_ECLAT, order=o) for o in orders]
+    for a, b in list(zip(free, tight))[:2]:
+        assert all(np.array_equal(getattr(a, x), getattr(b, x)) for x in ("offsets", "items", "supports"))
+    sets = [{tuple(r.items[r.offsets[k]:r.offsets[k + 1]].tolist()) for k in range(len(r))} for r in (free[2], tight[2])]
+    assert sets[0] == sets[1] and len(sets[1]) == len(tight[2])
+
+
+def test_batches_ordered_by_the_host(oracle_lib, limits):
+    from cupami_b200 import cuEclat
+
+    csrs = [_csr(30000, 500, 12), _csr(900, 60, 5), _csr(50000, 200, 20)]
+    limits(order_bytes=1)
+    for csr, m in zip(csrs, cuEclat.mineBatch(csrs, 0.004)):
+        want = oracle_lib.to_dict(*oracle_lib.mine_csr(csr.offsets, csr.items, 0.004))
+        assert list(m.getPatterns().items()) == list(want.items())
+
+
 # Thresholds that itemsets of no transaction pass: baskets of one item (frames without a row below
 # the classes), two items that occur among eleven that do not, and a database without transactions.
 @pytest.mark.parametrize("minsup", [0, -3])

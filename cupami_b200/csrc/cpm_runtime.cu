@@ -44,6 +44,7 @@
 
 using namespace cpm;
 
+#include "rt_hostpool.inc"
 #include "rt_context.inc"
 #include "rt_database.inc"
 #include "rt_pairs.inc"

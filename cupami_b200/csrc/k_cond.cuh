@@ -627,7 +627,6 @@ __global__ void __launch_bounds__(COND_BLOCK) k_cond_emit(CondParams P) {
                 u.ab = s_ab;
                 u.idx_words = form.idx_words;
                 u.frame = s_fid;
-                atomicAdd(&st->bytes_alg, 8ull * form.words);
             }
         }
         __syncthreads();
@@ -734,8 +733,11 @@ __global__ void __launch_bounds__(COND_BLOCK) k_cond_publish(CondParams P) {
         const bool bits = u.form == 2;
         const uint32_t R = bits ? u.next : u.rows;
         if ((long long)R < f.minsup) continue;  // no two survivors meet often enough
-        if (tid == 0)
+        if (tid == 0) {
             cond_frame(P, f, bits, u.frame, u.mb, ns, u.ab, u.idx_words, max(1u, (u.n + 127u) / 128u), R, u.next);
+            // What the child frame holds: its bitsets, or row elements and an occurrence for each but a row's last.
+            atomicAdd(&st->bytes_alg, bits ? 16ull * ns * max(1u, (R + 127u) / 128u) : 2ull * u.next + 8ull * (u.next - R));
+        }
         // Chunks of members: occurrences, then a unit for each that has enough for a child.
         for (uint32_t r0 = 0; r0 < ns; r0 += COND_BLOCK) {
             const uint32_t r = r0 + tid;

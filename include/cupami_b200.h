@@ -117,9 +117,10 @@ typedef struct {
     uint64_t frames;               /* deep equivalence classes processed */
     uint64_t work_items;           /* (frame, position) units processed */
     uint64_t intersections;        /* sibling AND+popcount operations */
-    uint64_t bytes_alg;            /* sum over units of 8*W*(1 + siblings + survivors) */
-    uint64_t pair_ops;             /* tensor ops issued by the pair Gram (2*K*rows*cols; 0: pairs counted
-                                      on CUDA cores or from the rows) */
+    uint64_t bytes_alg;            /* sum over units of 8*W*(1 + siblings + survivors); conditional rows: 8 per
+                                      occurrence and 2 per row element met, and what child frames hold */
+    uint64_t pair_ops;             /* operations of the pair Gram (2*K*rows*cols; 0: pairs counted from
+                                      the rows) */
     uint64_t kernel_launches;
     uint64_t retries;              /* arena/queue overflow retries (failed rounds included) */
     uint64_t deep_rounds;          /* memory-bounded rounds of the deep phase (0: one launch) */

@@ -158,6 +158,21 @@ def test_batches_ordered_by_the_host(oracle_lib, limits):
         assert list(m.getPatterns().items()) == list(want.items())
 
 
+# Occurrences of all databases together above the limit (26 MB), each database's below it; small
+# ids, and ids that take one database after the other anyhow.
+@pytest.mark.parametrize("step", [1, 1 << 19])
+def test_batches_whose_occurrences_do_not_fit_at_once(oracle_lib, limits, step):
+    from cupami_b200 import TransactionCSR, cuEclat
+
+    csrs = [_csr(n, 200, 12) for n in (120001, 140001, 160001, 120002)]
+    csrs = [TransactionCSR(c.offsets, c.items * np.uint32(step), c.universe * step) for c in csrs]
+    limits(alloc_bytes=14 << 20, arena_bytes=12 << 20)
+    miners = cuEclat.mineBatch(csrs, 0.2)
+    for csr, m in zip(csrs, miners):
+        want = oracle_lib.to_dict(*oracle_lib.mine_csr(csr.offsets, csr.items, 0.2))
+        assert len(want) > 3 and list(m.getPatterns().items()) == list(want.items())
+
+
 # Thresholds that itemsets of no transaction pass: baskets of one item (frames without a row below
 # the classes), two items that occur among eleven that do not, and a database without transactions.
 @pytest.mark.parametrize("minsup", [0, -3])

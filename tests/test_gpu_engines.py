@@ -28,3 +28,17 @@ def test_bytes_of_conditional_rows(size, per_basket):
     assert s["n_patterns"] == 13 + 78 + (286 if size == 3 else 0)
     assert s["row_units"] == s["work_items"] and (size == 2 or s["row_units"] > 0)
     assert s["bytes_alg"] == per_basket * n
+
+
+# The dispatch by work: pairs counted from the rows or multiplied, deep levels over conditional rows
+# (all of their units below the classes) or over tidsets (root units of the classes besides).
+@pytest.mark.parametrize("n,items,mean,minsup,row_pairs,rows", [
+    (4097, 700, 6, 12, True, False), (8191, 300, 15, 60, True, True), (16385, 400, 30, 480, False, False),
+    (70001, 600, 60, 7000, False, False), (20000, 2500, 12, 30, True, True), (131073, 90, 4, 150, True, True),
+    (2048, 500, 50, 150, False, False), (400000, 200, 20, 4000, False, True)])
+def test_engine_by_work(n, items, mean, minsup, row_pairs, rows):
+    rng = np.random.default_rng(n)
+    w = 1.0 / np.arange(1, items + 1) ** 0.9
+    s = _mined(rng.random((n, items)) < np.minimum(0.97, w * mean / w.sum()), minsup)
+    assert (s["pair_ops"] == 0) == row_pairs
+    assert s["work_items"] > 0 and (s["work_items"] == s["projected_units"] + s["row_units"]) == rows

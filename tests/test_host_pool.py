@@ -41,6 +41,16 @@ int main() {
     WANT(live <= 5);
     { auto a = pool->take(500 * MB), c = pool->take(450 * MB); WANT(a->p != c->p); }
     { auto a = pool->take(600 * MB); WANT(!a->pinned); }
+    {   // page-locked memory stops at 2 GB, whatever is held
+        std::vector<std::shared_ptr<HostBlock>> held;
+        size_t pinned = 0;
+        for (int k = 0; k < 40; ++k) {
+            held.push_back(pool->take(100 * MB));
+            pinned += held.back()->pinned ? held.back()->bytes : 0;
+        }
+        WANT(pinned > 1900 * MB && pinned <= 2048 * MB && !held.back()->pinned);
+    }
+    { auto a = pool->take(100 * MB); WANT(a->pinned); }
     full = true;
     { auto a = pool->take(3 * MB); WANT(!a->pinned); }
     pool.reset();

@@ -14,18 +14,18 @@ def _mined(held, minsup):
     return db.mine(minsup, _native.CPM_ECLAT).stats
 
 
-# Baskets of exactly two or three of 13 items, every pair and triple frequent.  No frame survives below
+# Baskets of exactly two or three of 40 items, every pair and triple frequent.  No frame survives below
 # the pairs of two items.  Of three, each basket is one row of the class of its first item (two
 # elements, one of them listed: 12 bytes), and is met once more by its first two items' unit (an
 # occurrence and an element: 10 bytes); no basket is left below those.
 @pytest.mark.parametrize("size,per_basket", [(2, 0), (3, 22)])
 def test_bytes_of_conditional_rows(size, per_basket):
-    n, items = 1_900_000, 13
+    n, items = 1_000_000, 40
     rng = np.random.default_rng(size)
     held = np.zeros((n, items), bool)
     np.put_along_axis(held, np.argsort(rng.random((n, items)), axis=1)[:, :size], True, axis=1)
-    s = _mined(held, 100)
-    assert s["n_patterns"] == 13 + 78 + (286 if size == 3 else 0)
+    s = _mined(held, 40)
+    assert s["n_patterns"] == 40 + 780 + (9880 if size == 3 else 0)
     assert s["row_units"] == s["work_items"] and (size == 2 or s["row_units"] > 0)
     assert s["bytes_alg"] == per_basket * n
 
@@ -33,9 +33,11 @@ def test_bytes_of_conditional_rows(size, per_basket):
 # The dispatch by work: pairs counted from the rows or multiplied, deep levels over conditional rows
 # (all of their units below the classes) or over tidsets (root units of the classes besides).
 @pytest.mark.parametrize("n,items,mean,minsup,row_pairs,rows", [
-    (4097, 700, 6, 12, True, False), (8191, 300, 15, 60, True, True), (16385, 400, 30, 480, False, False),
+    (4097, 700, 6, 12, True, False), (8191, 300, 15, 60, True, True), (16385, 400, 30, 480, False, True),
     (70001, 600, 60, 7000, False, False), (20000, 2500, 12, 30, True, True), (131073, 90, 4, 150, True, True),
-    (2048, 500, 50, 150, False, False), (400000, 200, 20, 4000, False, True)])
+    (2048, 500, 50, 150, False, False), (400000, 200, 20, 1600, False, True),
+    # long tidsets and few candidates: rows measured 1.5 to 4 times slower than the walk
+    (400000, 200, 20, 4000, False, False), (600000, 60, 4, 6000, True, False), (600000, 200, 6, 3600, True, False)])
 def test_engine_by_work(n, items, mean, minsup, row_pairs, rows):
     rng = np.random.default_rng(n)
     w = 1.0 / np.arange(1, items + 1) ** 0.9

@@ -53,7 +53,7 @@ class _Mines:
 # Steps of less than the fifth that remembered sizes add: one of the budgets is filled to over
 # four fifths, and those below overflow (frames of bitsets alone, and frames of rows).
 @pytest.mark.parametrize("n,items,mean,minsup,most,least", [(20000, 2500, 12, 30, 8 << 20, 176 << 10),
-                                                            (400000, 200, 20, 4000, 1300 << 20, 48 << 20)])
+                                                            (400000, 200, 20, 1600, 1300 << 20, 48 << 20)])
 def test_mines_of_one_database_under_shrinking_arenas(oracle_lib, limits, n, items, mean, minsup, most, least):
     mines = _Mines(oracle_lib, _csr(n, items, mean), minsup)
     stats = []
@@ -68,7 +68,7 @@ def test_mines_of_one_database_under_shrinking_arenas(oracle_lib, limits, n, ite
 def test_a_search_that_overflows_both_engines_is_mined_again(oracle_lib, limits):
     """Rows, then tidsets, overflow the same arena; the next mines go in rounds from the start."""
     limits(arena_bytes=64 << 20)
-    mines = _Mines(oracle_lib, _csr(400001, 200, 20), 4000)
+    mines = _Mines(oracle_lib, _csr(400001, 200, 20), 1600)
     first, *rest = [mines.again() for _ in range(3)]
     assert first["retries"] >= 1 and all(s["deep_rounds"] > 0 for s in (first, *rest))
 
@@ -85,7 +85,7 @@ def test_a_walk_over_tidsets_does_not_steer_conditional_rows(oracle_lib, limits)
 
 @pytest.mark.parametrize("units", [1, 40, 100])
 def test_levels_outgrow_their_tables(oracle_lib, limits, units):
-    mines = _Mines(oracle_lib, _csr(400002, 200, 20), 4000)
+    mines = _Mines(oracle_lib, _csr(400002, 200, 20), 1600)
     free = mines.again()
     limits(level_units=units)
     stats = [mines.again(), mines.again()]
@@ -93,12 +93,12 @@ def test_levels_outgrow_their_tables(oracle_lib, limits, units):
     assert all(s["retries"] > 0 and s["row_units"] == free["row_units"] for s in stats)
 
 
-# No room for the conditional rows (their occurrences take 12 MB); the tables of a search with
+# No room for the conditional rows (their occurrences take 25 MB); the tables of a search with
 # them (frames: 9.0 MB); the counters of their levels (2 GB).  Each time there is for the walk.
 @pytest.mark.parametrize("shape,limit", [
-    ((400003, 60, 4, 20000), {"arena_bytes": 8 << 20, "alloc_bytes": 8 << 20}),
+    ((800000, 60, 4, 8000), {"arena_bytes": 20 << 20, "alloc_bytes": 20 << 20}),
     ((20000, 2500, 12, 30), {"arena_bytes": 8 << 20, "alloc_bytes": 17 << 19}),
-    ((400003, 200, 20, 4000), {"arena_bytes": 1 << 30, "alloc_bytes": 1200 << 20, "level_units": 1 << 20})])
+    ((400003, 200, 20, 1600), {"arena_bytes": 1 << 30, "alloc_bytes": 1200 << 20, "level_units": 1 << 20})])
 def test_searches_go_on_without_the_memory_they_were_planned_with(oracle_lib, limits, shape, limit):
     n, items, mean, minsup = shape
     mines = _Mines(oracle_lib, _csr(n, items, mean), minsup)
@@ -174,13 +174,13 @@ def test_batches_whose_occurrences_do_not_fit_at_once(oracle_lib, limits, step):
 
 
 # Thresholds that itemsets of no transaction pass: baskets of one item (frames without a row below
-# the classes), two items that occur among eleven that do not, and a database without transactions.
+# the classes), two items that occur among fourteen that do not, and a database without transactions.
 @pytest.mark.parametrize("minsup", [0, -3])
 @pytest.mark.parametrize("kind", ["single", "pair", "none"])
 def test_levels_whose_units_have_no_occurrences(kind, minsup):
     from cupami_b200 import _native
 
-    items, n = 13, 0 if kind == "none" else 1_900_000
+    items, n = 16, 0 if kind == "none" else 1_900_000
     rng = np.random.default_rng(items)
     held = np.zeros((n, items), bool)
     if kind == "single":

@@ -33,9 +33,11 @@ def test_bytes_of_conditional_rows(size, per_basket):
 # The dispatch by work: pairs counted from the rows or multiplied, deep levels over conditional rows
 # (all of their units below the classes) or over tidsets (root units of the classes besides).
 @pytest.mark.parametrize("n,items,mean,minsup,row_pairs,rows", [
-    (4097, 700, 6, 12, True, False), (8191, 300, 15, 60, True, True), (16385, 400, 30, 480, False, True),
+    (4097, 700, 6, 12, False, False), (8191, 300, 15, 60, True, True), (16385, 400, 30, 480, False, True),
     (70001, 600, 60, 7000, False, False), (20000, 2500, 12, 30, True, True), (131073, 90, 4, 150, True, True),
     (2048, 500, 50, 150, False, False), (400000, 200, 20, 1600, False, True),
+    # too short a search for its rows to be used again (uniform 10,000 x 50)
+    (10000, 50, 6, 100, False, False),
     # long tidsets and few candidates: rows measured 1.5 to 4 times slower than the walk
     (400000, 200, 20, 4000, False, False), (600000, 60, 4, 6000, True, False), (600000, 200, 6, 3600, True, False)])
 def test_engine_by_work(n, items, mean, minsup, row_pairs, rows):

@@ -46,3 +46,22 @@ def test_engine_by_work(n, items, mean, minsup, row_pairs, rows):
     s = _mined(rng.random((n, items)) < np.minimum(0.97, w * mean / w.sum()), minsup)
     assert (s["pair_ops"] == 0) == row_pairs
     assert s["work_items"] > 0 and (s["work_items"] == s["projected_units"] + s["row_units"]) == rows
+
+
+# Batches: a CTA per item and database costs small databases more than the Gram of them all; of
+# tall databases over few items, whose Gram tiles are long, it costs less.
+@pytest.mark.parametrize("databases,n,items,mean,row_pairs", [(100, 3000, 60, 6, False), (120, 150_000, 40, 3, True)])
+def test_pairs_of_batches(databases, n, items, mean, row_pairs):
+    from cupami_b200 import _native
+
+    ctx = _native.context(0)
+    rng = np.random.default_rng(n)
+    w = 1.0 / np.arange(1, items + 1) ** 0.9
+    held = rng.random((n, items)) < np.minimum(0.97, w * mean / w.sum())
+    offsets = np.zeros(n + 1, dtype=np.uint64)
+    np.cumsum(held.sum(axis=1), out=offsets[1:])
+    cols = np.nonzero(held)[1].astype(np.uint32)
+    dbs = _native.Database.from_ids_batch(ctx, [(offsets, cols)] * databases)
+    found = _native.mine_batch(ctx, dbs, [n // 50] * databases)
+    assert (found[0].stats["pair_ops"] == 0) == row_pairs
+    assert all(np.array_equal(r.items, found[0].items) and np.array_equal(r.supports, found[0].supports) for r in found)

@@ -137,7 +137,10 @@ constexpr unsigned REF_UNROLL = 8;
 // 4 bytes a lane, whole lines a warp.  Bound by L2: 65,536 pairs over 1,000
 // rows of 3,125 words read 1.6 GB from it in 103 us (342 us with one load of
 // each row at a time).  WIDTH 2, the pair batches of the drivers, is unrolled.
-template <unsigned WIDTH>
+// UNROLL words are in flight, as many as rows of up to 32 and 64 words fill
+// (one and two); with eight for those too, 60,000 candidates of four rows took
+// 28.7 us for 20 (7 words) and 29.2 for 23 (33 words).
+template <unsigned WIDTH, unsigned UNROLL>
 __global__ void __launch_bounds__(256) k_ref_count(const uint32_t *__restrict__ bits, uint64_t words,
                                                    const uint32_t *__restrict__ cand, uint64_t n, uint32_t width,
                                                    unsigned long long *__restrict__ support) {
@@ -147,20 +150,26 @@ __global__ void __launch_bounds__(256) k_ref_count(const uint32_t *__restrict__ 
     const uint32_t w_n = WIDTH ? WIDTH : width;
     const uint32_t *cc = cand + warp * w_n;
     unsigned long long s = 0;
-    for (uint64_t w0 = lane; w0 < words; w0 += 32 * REF_UNROLL) {
-        uint32_t acc[REF_UNROLL];
+    if (UNROLL == 1)
+        for (uint64_t w = lane; w < words; w += 32) {
+            uint32_t acc = 0xffffffffu;
+            for (uint32_t j = 0; j < w_n; ++j) acc &= __ldg(bits + (uint64_t)cc[j] * words + w);
+            s += __popc(acc);
+        }
+    for (uint64_t w0 = lane; UNROLL > 1 && w0 < words; w0 += 32 * UNROLL) {
+        uint32_t acc[UNROLL];
         const uint32_t *row = bits + (uint64_t)__ldg(cc) * words;
 #pragma unroll
-        for (unsigned u = 0; u < REF_UNROLL; ++u) acc[u] = w0 + 32 * u < words ? __ldg(row + w0 + 32 * u) : 0u;
+        for (unsigned u = 0; u < UNROLL; ++u) acc[u] = w0 + 32 * u < words ? __ldg(row + w0 + 32 * u) : 0u;
 #pragma unroll
         for (uint32_t j = 1; j < w_n; ++j) {
             row = bits + (uint64_t)__ldg(cc + j) * words;
 #pragma unroll
-            for (unsigned u = 0; u < REF_UNROLL; ++u)
+            for (unsigned u = 0; u < UNROLL; ++u)
                 acc[u] &= w0 + 32 * u < words ? __ldg(row + w0 + 32 * u) : 0u;
         }
 #pragma unroll
-        for (unsigned u = 0; u < REF_UNROLL; ++u) s += __popc(acc[u]);
+        for (unsigned u = 0; u < UNROLL; ++u) s += __popc(acc[u]);
     }
     s = warp_sum_u64(s);
     if (!lane) support[warp] = s;

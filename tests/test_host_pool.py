@@ -36,6 +36,9 @@ int main() {
     { auto a = pool->take(380 * MB); WANT(a->p == big && made == 2); }
     { auto a = pool->take(MB); auto c = pool->take(100 * 1024); WANT(a->p != small->p && !c->pinned && made == 3); }
     { auto a = pool->take(MB); WANT(made == 3); }
+    // kept blocks of up to 128 MB serve any smaller request
+    { auto a = pool->take(100 * MB); WANT(made == 4); }
+    { auto a = pool->take(3 * MB), c = pool->take(40 * MB); WANT(made <= 5 && a->p != c->p); }
     // kept: at most four, of 512 MB together
     for (size_t mb : {8, 32, 128, 500, 2}) pool->take(mb * MB);
     WANT(live <= 5);
@@ -52,7 +55,7 @@ int main() {
     }
     { auto a = pool->take(100 * MB); WANT(a->pinned); }
     full = true;
-    { auto a = pool->take(3 * MB); WANT(!a->pinned); }
+    { auto a = pool->take(300 * MB); WANT(!a->pinned); }
     pool.reset();
     WANT(live == 1);
     small.reset();

@@ -171,14 +171,14 @@ class ClockSampler:
                 "samples": len(sm), "reasons": sorted(reasons)}
 
 
-def deep_traffic(workload, tidsets, arena_mb):
-    """The committed ncu record of one k_deep launch of this workload (DRAM
-    bytes per launch, L2 throughput), or None if there is none."""
+def deep_traffic(workload, tidsets, arena_mb, engine):
+    """The committed ncu record of one deep phase of this workload on this engine
+    ("rows": conditional rows, "walk": over tidsets) -- DRAM and L2 bytes --, or None."""
     p = ROOT / "profiles" / "k_deep_traffic.json"
     if not p.exists() or arena_mb:
         return None
     d = json.loads(p.read_text()).get(workload)
-    if not d or d.get("tidsets", 0) != tidsets:
+    if not d or d.get("tidsets", 0) != tidsets or d.get("engine", "walk") != engine:
         return None
     return d
 
@@ -908,12 +908,13 @@ def run_ours(args, world, rank, local):
         row_units = statistics.mean(sum(s.get("row_units", 0) for s in st) for st in eclat_stats)
         units = statistics.mean(sum(s.get("work_items", 0) for s in st) for st in eclat_stats)
         achieved = deep_bytes / (deep_ms * 1e-3) / 1e9 if deep_ms else 0.0
-        # The committed record is of the tidset walk; pairs counted from the rows mean the other engine ran.
-        tr = deep_traffic(args.workload, args.tidsets, args.arena_mb) if all(
-            s["pair_ops"] for st in eclat_stats for s in st) else None
+        # Over conditional rows every unit below the classes is a row or a projected one.
+        engine = "rows" if all(s["work_items"] == s["projected_units"] + s["row_units"]
+                               for st in eclat_stats for s in st) else "walk"
+        tr = deep_traffic(args.workload, args.tidsets, args.arena_mb, engine)
         traffic = tr["dram_bytes_per_launch"] if tr else None
         roof = {"kernel": "deep phase: conditional rows (k_cond_*) or k_deep, then k_local (a warp per projected unit)",
-                "bound": deep_bound(traffic, deep_bytes),
+                "bound": (tr or {}).get("bound") or deep_bound(traffic, deep_bytes), "engine": engine,
                 "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm, "traffic": traffic,
                 "peak_source": src, "frac_of": "HBM copy bandwidth (" + src + "); algorithmic bytes / kernel time",
                 "frac_of_8tbs_spec": achieved / 8000.0,

@@ -36,9 +36,10 @@
 // the buffers and reruns; nothing here waits.
 //
 // Measured (deep phase, k_local included; before: k_deep over tidsets in column
-// order): 1M x 20k 347 -> 29 ms (145 ms with rows but in column order), 250k x
-// 20k 37 -> 5.5 ms, 512 databases of 200 items 15.2 -> 7.2 ms, 2M x 400 3.2 ->
-// 2.1 ms, planted 100k x 1,000 0.227 -> 0.184 ms.
+// order): 1M x 20k 347 -> 23.5 ms, 250k x 20k 37 -> 3.5 ms, 512 databases of 200
+// items 15.2 -> 7.1 ms, planted 100k x 1,000 0.227 -> 0.143 ms.  Long tidsets over
+// few items are left to k_deep, in order of support (cond_plan): a mine of 2.4M
+// x 500 takes 4.3 ms in column order, 3.2 over rows and 1.5 so.
 #pragma once
 #include "k_batch.cuh"
 #include "k_deep.cuh"
@@ -636,6 +637,8 @@ __global__ void __launch_bounds__(COND_BLOCK) k_cond_emit(CondParams P) {
     }
 }
 
+// Bound by instruction issue: 74% of the issue slots busy at the classes of 250k
+// x 20k (0.85 ms; L2 29%, DRAM 2% of peak), 63% of the warps active.
 __global__ void __launch_bounds__(COND_BLOCK, 3) k_cond_write(CondParams P) {
     extern __shared__ uint32_t sm[];
     __shared__ uint32_t s_len, s_rows;

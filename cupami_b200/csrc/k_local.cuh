@@ -27,7 +27,9 @@
 // queued or running than keep the grid busy, child frames and what is left on
 // the stack go to the queue instead, for any warp.
 //
-// What bounds it: the latency of L2 and DRAM under load.  More warps lose
+// What bounds it: the latency of L2 and DRAM under load (250k x 20k: long
+// scoreboard the first stall, 41% of the issue slots busy, L2 34% and DRAM 22%
+// of peak, all 16 warps per SM that the registers allow).  More warps lose
 // more to each other's evictions than they hide: 1M x 20,000 sparse rows
 // (3.2M units, tidsets of 2.7 KB on average) take 7.5 ms with 16 warps per SM
 // (128 registers), 8.8 with 12, 8.6 with 20, 9.9 with 24 and 11.5 with 32;

@@ -90,8 +90,8 @@ typedef struct {
     int32_t  deep_ctas_per_sm;     /* resident deep-level CTAs per SM, 1-4 (capped by occupancy); 0 = automatic */
     int32_t  autotune;             /* 1: use the launch shape cpm_autotune found for this tidset length */
     /* With tidsets, list_div, deep_*, arena_bytes and collect_trace all 0, searches of some size are
-       mined in order of increasing support over conditional rows; what follows is then the walk over
-       tidsets of the others (any option set selects that walk, in column order). */
+       mined in order of increasing support, sparse ones over conditional rows; what follows is then
+       the walk over tidsets of the others (any option set selects that walk, in column order). */
     int32_t  tidsets;              /* deep-level tidset forms.  0: bitsets, plus transaction-id lists for
                                       tidsets held by under 1/32 of the transactions when a database's
                                       frequent bitsets exceed half the L2 and one bitset fits in shared
@@ -202,7 +202,8 @@ int  cpm_mine(cpm_ctx *ctx, cpm_db *db, int64_t min_sup, int algo,
 /* Eclat over many independent databases in one pass: one launch per stage
  * and one persistent deep-level launch for the whole batch.  out[d] is the
  * result of dbs[d] at min_sups[d], equal to cpm_mine(dbs[d], min_sups[d],
- * CPM_ECLAT); each result's statistics are those of the whole batch.  The
+ * CPM_ECLAT); each result's statistics are those of the whole batch, and the
+ * results may share memory, which is given back with the last of them.  The
  * reference mines one database per call (cuEclat.py:168-203). */
 int  cpm_mine_batch(cpm_ctx *ctx, cpm_db **dbs, uint32_t n_db, const int64_t *min_sups,
                     const cpm_opts *opts, cpm_result **out);

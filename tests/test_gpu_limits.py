@@ -194,6 +194,8 @@ def test_levels_whose_units_have_no_occurrences(kind, minsup):
     r = db.mine(minsup, _native.CPM_ECLAT)
     got = {tuple(r.items[r.offsets[k]:r.offsets[k + 1]].tolist()): s for k, s in enumerate(r.supports.tolist())}
     assert len(got) == len(r) == 2**items - 1
+    if n:  # over conditional rows
+        assert r.stats["work_items"] == r.stats["projected_units"] + r.stats["row_units"] > 0
     occur = {(i,): int(held[:, i].sum()) for i in range(items)}
     occur[4, 9] = int((held[:, 4] & held[:, 9]).sum())
     assert all(s == occur.get(p, 0) for p, s in got.items())
